@@ -36,6 +36,7 @@ int fail(acum_ctx* ctx, int code, const std::string& msg)
 
 int cuda_fail(acum_ctx* ctx, cudaError_t e, const char* what)
 {
+    (void)cudaGetLastError();  // reported here: not what a later launch has to find
     return fail(ctx, e == cudaErrorMemoryAllocation ? ACUM_ERR_NOMEM : ACUM_ERR_CUDA,
                 std::string(what) + ": " + cudaGetErrorString(e));
 }
@@ -801,6 +802,7 @@ Dropin* dropin_for(int dev, int kind)
     void* p = nullptr;
     if (cudaHostAlloc(&p, sizeof(DropinFacts) + sizeof(DeviceErr), cudaHostAllocPortable | cudaHostAllocMapped) !=
         cudaSuccess) {
+        (void)cudaGetLastError();
         acum_destroy(d->c);
         return nullptr;
     }

@@ -78,6 +78,7 @@ int bfail(acum_batch* b, int code, const std::string& msg)
 
 int bcuda(acum_batch* b, cudaError_t e, const char* what)
 {
+    (void)cudaGetLastError();  // reported here: not what a later launch has to find
     return bfail(b, ACUM_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 

@@ -36,6 +36,26 @@ struct DBuf {
     }
 };
 
+// Waits for a stream on every way out of a scope: declared behind what the stream's work writes
+// to (a host function's own variables, buffers that the next call takes), so that none of it is
+// given up with that work in flight.
+struct InFlight {
+    cudaStream_t s;
+    bool on = true;
+    explicit InFlight(cudaStream_t st) : s(st) {}
+    cudaError_t wait()
+    {
+        on = false;
+        return cudaStreamSynchronize(s);
+    }
+    ~InFlight()
+    {
+        if (on) cudaStreamSynchronize(s);
+    }
+    InFlight(const InFlight&) = delete;
+    InFlight& operator=(const InFlight&) = delete;
+};
+
 // NVTX range over one ABI call (visible in Nsight timelines; a no-op otherwise)
 struct NvtxRange {
     explicit NvtxRange(const char* name) { nvtxRangePushA(name); }

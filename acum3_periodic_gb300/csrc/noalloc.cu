@@ -21,8 +21,9 @@
 //    within the same tolerance) and refuses the others with the same status;
 //  * the first call on a device looks up the array's device address (cudaGetSymbolAddress)
 //    with that device current; make that first call before any stream capture;
-//  * every call synchronises `stream` before it returns: it reads a summary of E, vInf, tObs
-//    and the observers back to the host, and after the kernels the device error word;
+//  * every call that launched anything synchronises `stream` before it returns, whatever it
+//    returns: the summary of E, vInf, tObs and the observers and, after the kernels, the device
+//    error word go to variables of the call itself;
 //  * every call reuses the same array and leaves its contents behind; the call clears
 //    what must start at zero itself, and two calls whose GPU work overlaps (different
 //    streams or threads without ordering) race on the array -- serialise them;
@@ -95,6 +96,7 @@ extern "C" int acum_find_pressure_time_history_noalloc(const float* rObs, const 
         scratch = g_na_ptr[dev];
     }
     cudaStream_t st = (cudaStream_t)stream;
+    (void)cudaGetLastError();  // an earlier call's failure is not this one's
     // what the host needs of the device arrays in one read (through the start of the scratch);
     // the kernel bins on the uniform grid main.cu:124 builds: another tObs is refused, with the
     // tolerance of the allocating drop-in
@@ -102,11 +104,13 @@ extern "C" int acum_find_pressure_time_history_noalloc(const float* rObs, const 
     int host_memory = 0;
     cudaDeviceGetAttribute(&host_memory, cudaDevAttrPageableMemoryAccess, dev);
     DropinFacts facts;
+    DeviceErr h;
+    InFlight flight(st);  // nothing below returns with the device still writing to the two
     DropinFacts* const to = host_memory ? &facts : (DropinFacts*)scratch;
     if (launch_dropin_facts(false, E, nSurf, vInf, tObs, nTime, dPsi, rObs, nObs, to, st) != cudaSuccess ||
         (!host_memory &&
          cudaMemcpyAsync(&facts, scratch, sizeof(facts), cudaMemcpyDeviceToHost, st) != cudaSuccess) ||
-        cudaStreamSynchronize(st) != cudaSuccess)
+        flight.wait() != cudaSuccess)
         return bad(ACUM_ERR_CUDA, "findPressureTimeHistory_noalloc: reading E/vInf/tObs/rObs failed");
     if (facts.uneven) return bad(ACUM_ERR_UNSUPPORTED, "findPressureTimeHistory_noalloc: tObs must be t*dPsi");
     if (facts.negative) return bad(ACUM_ERR_INVALID, "findPressureTimeHistory_noalloc: negative element count");
@@ -135,8 +139,33 @@ extern "C" int acum_find_pressure_time_history_noalloc(const float* rObs, const 
         return bad(ACUM_ERR_INVALID, "findPressureTimeHistory_noalloc: no room for the error word");
     DeviceErr* derr = reinterpret_cast<DeviceErr*>(reinterpret_cast<unsigned char*>(scratch) + err_off);
     unsigned* rmax = reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(derr) + err_bytes - 16);
+    int sms = 0, optin = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    TonalRun r;
+    memset(&r, 0, sizeof(r));
+    r.g.E = (int)Et;
+    r.g.Epad = (int)Epad;
+    r.g.T = nTime;
+    r.g.nW = nW;
+    const int pass = nObs < kAnchorsMax ? nObs : kAnchorsMax;
+    r.g.O = pass;
+    r.g.a0 = a0;
+    r.g.rho = rhoRef;
+    r.g.oM = oM;
+    r.g.dPsi = dPsi;
+    r.g.dTau = dTau;
+    r.g.lpi = nTime * (double)dPsi;
+    const double* vi = facts.vinf;
+    for (int q = 0; q < 3; ++q) r.g.vinf[q] = vi[q];
+    r.g.obs_rmin = obs_rmin;
+    r.precision = ACUM_MIXED;
+    r.rmax = rmax;
+    if (plan_tonal(r, 0, 0, 0, sms, (size_t)optin) != cudaSuccess)
+        return bad(ACUM_ERR_UNSUPPORTED, "findPressureTimeHistory_noalloc: no tile shape fits this nTime");
     // the array keeps the previous call's contents: clear the sums, the error word and the
     // radius, which lie behind one another (the records kernel writes every slot)
+    flight.on = true;
     if (cudaMemsetAsync(acc, 0, err_off - acc_off + err_bytes, st) != cudaSuccess)
         return bad(ACUM_ERR_CUDA, "findPressureTimeHistory_noalloc: clearing scratch failed");
     AosArgs a;
@@ -158,33 +187,9 @@ extern "C" int acum_find_pressure_time_history_noalloc(const float* rObs, const 
     a.rho = rhoRef;
     a.rec32 = rec;
     a.rmax = rmax;
-    const double* vi = facts.vinf;
     Anchor* anc = reinterpret_cast<Anchor*>(reinterpret_cast<unsigned char*>(scratch) + kNoAllocBytes);
-    const int pass = nObs < kAnchorsMax ? nObs : kAnchorsMax;
     if (launch_aos_records(a, anchor_job(rObs, pass, nTime, a0, vi, oM, dPsi, anc), st) != cudaSuccess)
         return bad(ACUM_ERR_CUDA, "findPressureTimeHistory_noalloc: launch of the records kernel failed");
-    int sms = 0, optin = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    TonalRun r;
-    memset(&r, 0, sizeof(r));
-    r.g.E = (int)Et;
-    r.g.Epad = (int)Epad;
-    r.g.T = nTime;
-    r.g.nW = nW;
-    r.g.O = pass;
-    r.g.a0 = a0;
-    r.g.rho = rhoRef;
-    r.g.oM = oM;
-    r.g.dPsi = dPsi;
-    r.g.dTau = dTau;
-    r.g.lpi = nTime * (double)dPsi;
-    for (int q = 0; q < 3; ++q) r.g.vinf[q] = vi[q];
-    r.g.obs_rmin = obs_rmin;
-    r.precision = ACUM_MIXED;
-    r.rmax = rmax;
-    if (plan_tonal(r, 0, 0, 0, sms, (size_t)optin) != cudaSuccess)
-        return bad(ACUM_ERR_UNSUPPORTED, "findPressureTimeHistory_noalloc: no tile shape fits this nTime");
     r.rec = rec;
     r.anc = anc;
     r.acc = acc;
@@ -198,12 +203,11 @@ extern "C" int acum_find_pressure_time_history_noalloc(const float* rObs, const 
         if (le == cudaSuccess) le = plan_tonal(r, 0, 0, 0, sms, (size_t)optin);
         if (le == cudaSuccess) le = launch_tonal(r, st);
     }
-    DeviceErr h;
     if (le != cudaSuccess || launch_finalize(acc, nObs, nTime, pT, pL, pA, 2, st, r.err,
                                              host_memory ? (unsigned*)&h.bits : nullptr) != cudaSuccess)
         return bad(ACUM_ERR_CUDA, "findPressureTimeHistory_noalloc: launch failed");
     if ((!host_memory && cudaMemcpyAsync(&h, r.err, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess) ||
-        cudaStreamSynchronize(st) != cudaSuccess)
+        flight.wait() != cudaSuccess)
         return bad(ACUM_ERR_CUDA, "findPressureTimeHistory_noalloc: kernel failed");
     if (h.bits & ACUM_DEVERR_TIMEOUT) return bad(ACUM_ERR_TIMEOUT, "a bounded shared-memory pipeline wait ran out");
     return ACUM_OK;

@@ -1,0 +1,41 @@
+"""What the reference-shaped calls do after, and beside, calls that fail."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from acum3_periodic_gb300 import synth
+from oracle import oracle as O
+
+from test_dropin_gpu import call_dropin
+
+pytestmark = pytest.mark.gpu
+
+
+def _deck(k=0, **scale):
+    return synth.config_deck(0, replicate=700 + k, scale=dict(dict(n_span=2, n_chord_side=2, ntime=40, nobs=3), **scale))
+
+
+@pytest.mark.parametrize("name,dtype", [("noalloc", np.float32), ("", np.float32), ("f64", np.float64)])
+def test_after_a_failed_allocation(name, dtype):
+    """An allocation that failed on the same thread (the reason to turn to the allocation-free
+    entry point) is that call's error, not the next one's."""
+    torch = pytest.importorskip("torch")
+    from acum3_periodic_gb300 import native
+    L = native.lib()
+    fn = getattr(L, "_".join(["acum_find_pressure_time_history"] + [name] * bool(name)))
+    d = _deck()
+    f = O.preprocess(d)
+    rc, *ref = call_dropin(fn, d, f, dtype, torch)
+    assert rc == 0
+
+    def failed_first(*a):
+        p = C.c_void_p()
+        assert L.acum_host_alloc(C.byref(p), 1 << 60) != 0
+        return fn(*a)
+
+    rc, *got = call_dropin(failed_first, d, f, dtype, torch)
+    assert rc == 0
+    for a, b in zip(got, ref):
+        # the FP64 sums of several blocks add in any order
+        np.testing.assert_allclose(a, b, rtol=0, atol=1e-6 * np.abs(b).max())
