@@ -55,15 +55,26 @@ __host__ __device__ __forceinline__ int nwin32(int T) { return (T + kStride32 - 
 // sample's observer time lies from its step plus the observer's anchor (the retarded
 // time of the origin): |t - t0| <= |x| / (a0 - |vInf|), because the travel time through a
 // uniformly moving medium changes by at most 1 / (a0 - |vInf|) per unit of source
-// displacement; r = the records' largest |x|, kb = oM / dPsi bins per second.  1e30 when
-// r is not finite or the flight is not subsonic.
+// displacement; r = the records' largest |x|, kb = oM / dPsi bins per second.
+// ring_reach_rate: bins per unit of |x|, a normal float; -1 where there is no bound: flight
+// that is not subsonic, or a time that does not run forwards (kb <= 0).
+__host__ __device__ __forceinline__ double ring_reach_rate(double vx, double vy, double vz, double a0, double kb)
+{
+    const double vm = sqrt(vx * vx + vy * vy + vz * vz);
+    if (!(vm < 0.999 * a0)) return -1.0;
+    const double k = kb / (a0 - vm) * 1.0001;
+    return k >= 0x1p-126 && k < 0x1p127 ? k : -1.0;
+}
+// 1e30 when r is not finite or there is no bound
 __host__ __device__ __forceinline__ double ring_reach_bins(float r, double vx, double vy, double vz, double a0,
                                                            double kb)
 {
-    const double vm = sqrt(vx * vx + vy * vy + vz * vz);
-    if (!(r <= 1.0e30f) || !(vm < 0.999 * a0)) return 1.0e30;
-    return (double)r * kb / (a0 - vm) * 1.0001 + 2.0;
+    const double k = ring_reach_rate(vx, vy, vz, a0, kb);
+    if (!(r <= 1.0e30f) || k < 0.0) return 1.0e30;
+    return (double)r * k + 2.0;
 }
+// the same in FP32 for the kernels, k = (float)ring_reach_rate: a little larger for its rounding
+__host__ __device__ __forceinline__ float ring_reach_float(float r, float k) { return r * k * 1.000001f + 2.01f; }
 // Whether the ring kernel serves a deck: a ring of R slots holds every bin a window of 31
 // intervals can reach, and the observer-time offset of every sample is bounded by the
 // reach, so that the ring kernel needs no per-sample range check.  The second holds when
@@ -93,15 +104,22 @@ inline float ring_limit(double vx, double vy, double vz, double a0, double kb, d
         return ring_ok(r, vx, vy, vz, a0, kb, obs_rmin, R);
     };
     if (!ok(0)) return -1.f;
-    // the two bounds solved for r, then the last float that passes
+    // the two bounds solved for r, which a few roundings separate from the last float that
+    // passes; found between its neighbours, or between 0 and infinity where they do not hold it
     const double vm = sqrt(vx * vx + vy * vy + vz * vz);
-    double guess = (0.5 * (R - 40) - 2.0) * (a0 - vm) / (1.0001 * kb);
+    double guess = (0.5 * (R - 40) - 2.0) / ring_reach_rate(vx, vy, vz, a0, kb);
     if (vm > 0.0) guess = std::min(guess, sqrt(a0 * a0 - vm * vm) * obs_rmin / (1.01 * vm));
-    float g = (float)std::min(std::max(guess, 0.0), 1.0e30);
-    unsigned lo;
-    memcpy(&lo, &g, sizeof(lo));
-    while (!ok(lo)) --lo;
-    while (ok(lo + 1)) ++lo;
+    const float g = (float)std::min(std::max(guess, 0.0), 1.0e30);
+    unsigned at;
+    memcpy(&at, &g, sizeof(at));
+    unsigned lo = at > 4 ? at - 4 : 0, hi = at + 4;
+    if (!ok(lo)) lo = 0;
+    if (ok(hi)) hi = 0x7f800000u;
+    while (hi - lo > 1) {
+        const unsigned mid = lo + (hi - lo) / 2;
+        if (ok(mid)) lo = mid;
+        else hi = mid;
+    }
     float r;
     memcpy(&r, &lo, sizeof(r));
     return r;
@@ -330,7 +348,7 @@ struct KParams {
                             // each tests the records' reach
     const unsigned* rmax;   // mixed: the records' largest |x| (note_radius bits)
     float ring_max, ring_lo_max;  // mixed: the largest |x| of records that fit `ring`, `ring_lo` (ring_limit)
-    float reach_k;          // mixed: bins of reach per unit of |x| (ring_reach_bins)
+    float reach_k;          // mixed: bins of reach per unit of |x| (ring_reach_rate)
     const Anchor* anc;
     const double* obs64;
     // mixed constants, as pairs (both halves equal: the operands of the packed FP32
