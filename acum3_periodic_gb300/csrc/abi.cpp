@@ -835,8 +835,9 @@ int find_pth(const S* rObs, const S* tObs, S* pT, S* pL, S* pA, const S* Xham, c
     cudaStream_t st = stream_v ? (cudaStream_t)stream_v : (cudaStream_t)0;
     // the small per-surface arrays and the bin grid live in device memory, as the reference
     // passes them: what the host needs of them in one read
+    InFlight flight(st);
     CK(nullptr, launch_dropin_facts(f64, Ecnt, nSurf, vInf, tObs, nTime, dPsi, rObs, nObs, dr->facts, st));
-    CK(nullptr, cudaStreamSynchronize(st));
+    CK(nullptr, flight.wait());
     const DropinFacts facts = *dr->facts;
     if (facts.uneven) return fail(nullptr, ACUM_ERR_UNSUPPORTED, "findPressureTimeHistory: tObs must be t*dPsi");
     if (facts.negative) return fail(nullptr, ACUM_ERR_INVALID, "findPressureTimeHistory: negative element count");
@@ -845,6 +846,27 @@ int find_pth(const S* rObs, const S* tObs, S* pT, S* pL, S* pA, const S* Xham, c
     const int nW = (nTime + kWin - 1) / kWin;
     const int Epad = (int)((E + 7) / 8 * 8);
     const size_t nrec = f64 ? (size_t)Epad * nW * kGroups * kWin * 4 : (size_t)Epad * nwin32(nTime) * kGroups32 * kWin * 4;
+    TonalRun r;
+    memset(&r, 0, sizeof(r));
+    r.g.E = (int)E;
+    r.g.Epad = Epad;
+    r.g.T = nTime;
+    r.g.nW = nW;
+    r.g.O = nObs;
+    r.g.a0 = a0;
+    r.g.rho = rhoRef;
+    r.g.oM = oM;
+    r.g.dPsi = dPsi;
+    r.g.dTau = dTau;
+    r.g.lpi = nTime * dPsi;
+    for (int q = 0; q < 3; ++q) r.g.vinf[q] = facts.vinf[q];
+    r.g.obs_rmin = facts.obs_rmin;
+    r.precision = f64 ? ACUM_PLAIN_FP64 : ACUM_MIXED;
+    const size_t nsum = (size_t)nObs * nTime * 2;
+    // the records' largest |x| behind the bin sums: one clearing for both
+    CK(nullptr, c->d_acc.ensure(nsum + (f64 ? 0 : 1)));
+    r.rmax = f64 ? nullptr : reinterpret_cast<unsigned*>(c->d_acc.p + nsum);
+    CK(nullptr, plan_tonal(r, 0, 0, 0, c->num_sms, c->smem_optin));
     AosArgs a;
     memset(&a, 0, sizeof(a));
     a.X = Xham;
@@ -869,46 +891,26 @@ int find_pth(const S* rObs, const S* tObs, S* pT, S* pL, S* pA, const S* Xham, c
     } else {
         CK(nullptr, c->d_rec32.ensure(nrec));
         a.rec32 = c->d_rec32.p;
-        // the records' largest |x| behind the bin sums: one clearing for both
-        CK(nullptr, c->d_acc.ensure((size_t)nObs * nTime * 2 + 1));
-        CK(nullptr, cudaMemsetAsync(c->d_acc.p, 0, (size_t)nObs * nTime * 16 + 8, st));
-        a.rmax = reinterpret_cast<unsigned*>(c->d_acc.p + (size_t)nObs * nTime * 2);
+        CK(nullptr, c->d_anc.ensure((size_t)nObs));
+        a.rmax = reinterpret_cast<unsigned*>(c->d_acc.p + nsum);
     }
     AnchorJob job;
     memset(&job, 0, sizeof(job));
-    if (!f64) {
-        CK(nullptr, c->d_anc.ensure((size_t)nObs));
+    if (!f64)
         job = anchor_job(reinterpret_cast<const float*>(rObs), nObs, nTime, a0, facts.vinf, oM, dPsi, c->d_anc.p);
-    }
+    // from here on work is in flight on the workspaces
+    flight.on = true;
+    if (!f64 || r.t.nchunk > 1)
+        CK(nullptr, cudaMemsetAsync(c->d_acc.p, 0, nsum * 8 + (f64 ? 0 : 8), st));
     CK(nullptr, launch_aos_records(a, job, st));
-    TonalRun r;
-    memset(&r, 0, sizeof(r));
-    r.g.E = (int)E;
-    r.g.Epad = Epad;
-    r.g.T = nTime;
-    r.g.nW = nW;
-    r.g.O = nObs;
-    r.g.a0 = a0;
-    r.g.rho = rhoRef;
-    r.g.oM = oM;
-    r.g.dPsi = dPsi;
-    r.g.dTau = dTau;
-    r.g.lpi = nTime * dPsi;
-    for (int q = 0; q < 3; ++q) r.g.vinf[q] = facts.vinf[q];
-    r.g.obs_rmin = facts.obs_rmin;
-    r.precision = f64 ? ACUM_PLAIN_FP64 : ACUM_MIXED;
-    r.rmax = a.rmax;
-    CK(nullptr, plan_tonal(r, 0, 0, 0, c->num_sms, c->smem_optin));
     r.rec = f64 ? (const void*)c->d_rec64.p : (const void*)c->d_rec32.p;
     r.obs64 = f64 ? reinterpret_cast<const double*>(rObs) : nullptr;
     r.anc = f64 ? nullptr : c->d_anc.p;
-    if (f64) CK(nullptr, c->d_acc.ensure((size_t)nObs * nTime * 2));
     r.acc = c->d_acc.p;
     r.err = c->d_err.p;
-    if (f64 && r.t.nchunk > 1) CK(nullptr, cudaMemsetAsync(c->d_acc.p, 0, (size_t)nObs * nTime * 16, st));
     CK(nullptr, launch_tonal(r, st));
     CK(nullptr, launch_finalize(c->d_acc.p, nObs, nTime, pT, pL, pA, f64 ? 1 : 2, st, c->d_err.p, &dr->err->bits));
-    CK(nullptr, cudaStreamSynchronize(st));
+    CK(nullptr, flight.wait());
     if (dr->err->bits & ACUM_DEVERR_TIMEOUT) {
         cudaMemset(c->d_err.p, 0, sizeof(DeviceErr));
         return fail(nullptr, ACUM_ERR_TIMEOUT, "a bounded shared-memory pipeline wait ran out");
@@ -957,6 +959,7 @@ extern "C" int acum_preprocess_imper(float* Xham, float* Nham, float* Vham, floa
     if (!dr) return fail(nullptr, ACUM_ERR_CUDA, "preprocess_imper: cannot create a context");
     std::lock_guard<std::mutex> lock(dr->mu);
     acum_ctx* c = dr->c;
+    InFlight flight(c->stream);
     // surface rows from the AoS arrays (what read_surf stored, io.cu:318)
     std::vector<int> ne(E, E + nSurf);
     size_t tot = 0;
@@ -1181,6 +1184,7 @@ int preprocess_per_t(S* Xham, S* Nham, S* Vham, S* Uham, S* PRham, int nSurf, co
     cudaStream_t st = c->stream;
     S* host[5] = {Xham, Nham, Vham, Uham, PRham};
     PerBuffers b;
+    InFlight flight(st);
     for (int q = 0; q < 5; ++q) {
         CK(nullptr, cudaMalloc(&b.d[q], (size_t)L.extent[q] * sizeof(S)));
         CK(nullptr, cudaMemcpyAsync(b.d[q], host[q], (size_t)L.extent[q] * sizeof(S), cudaMemcpyHostToDevice, st));
@@ -1190,7 +1194,7 @@ int preprocess_per_t(S* Xham, S* Nham, S* Vham, S* Uham, S* PRham, int nSurf, co
     c->launches += 1;
     for (int q = 0; q < 5; ++q)
         CK(nullptr, cudaMemcpyAsync(host[q], b.d[q], (size_t)L.extent[q] * sizeof(S), cudaMemcpyDeviceToHost, st));
-    CK(nullptr, cudaStreamSynchronize(st));
+    CK(nullptr, flight.wait());
     return ACUM_OK;
 }
 

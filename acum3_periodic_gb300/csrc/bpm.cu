@@ -1316,9 +1316,12 @@ extern "C" int acum_find_bb_noise(int nSurf_BB, int nObs, int nTime, float dTau,
     acum_ctx* c = dr->c;
     DeviceGuard g(dev);
     BpmState* s = state(c);
+    InFlight flight(c->stream);
     const int rc = bb_noise(c, s, nSurf_BB, nObs, nTime, dTau, span, omega, ccw, psi_offset, trip, rotate, translate,
                             xsPtr, dsPtr, nsect, xyzcR, bbdata, nsect_t, nmach_t, naoa_t, nre_t, aPtr, mPtr, rPtr, sPtr,
                             dPtr, sect_t, mach_t, aoa_t, re_t, bbdata_t, t_del, vInf, rObs, a0, BBspl, BBoaspl);
+    if (rc == ACUM_OK) flight.on = false;  // it has waited
+    else flight.wait();
     // the workspaces stay for the next call unless they are large
     if (s->bytes() > kKeepBytes) release_bpm_state(c);
     return rc;

@@ -93,7 +93,8 @@ void release_bpm_state(struct ::acum_ctx* ctx);
 
 // The workspaces of the reference-shaped calls on one device, kept from call to call (their
 // buffers are scratch; nothing of a call's data is used by the next).  `mu` is held for the
-// whole call, which ends by waiting for its stream: one call at a time per device and kind.
+// whole call, every way out of which waits for its stream (InFlight): one call at a time per
+// device and kind.
 struct Dropin {
     std::mutex mu;
     struct ::acum_ctx* c = nullptr;
