@@ -76,6 +76,7 @@ struct BpmState {
                4 * (geo.n + sc.n + amp.n + fl.n + seed_f.n + out_f.n) + blob.n;
     }
     DBuf<float> geo, sc, amp;
+    int per_sm = 0;  // blocks of bb_obs_kernel that run on an SM at one time (0: not asked yet)
     bool uploaded = false;
 };
 
@@ -976,8 +977,10 @@ static int bpm_enqueue(acum_ctx* ctx, BBDev& d, int aa_mode, const float* seed_s
         return cuda_fail(ctx, e, "bpm alloc");
     if (!s->ff.p) {
         if ((e = s->ff.ensure(kBands)) != cudaSuccess ||
-            (e = cudaMemcpy(s->ff.p, kBandHz, kBands * 8, cudaMemcpyHostToDevice)) != cudaSuccess)
+            (e = cudaMemcpy(s->ff.p, kBandHz, kBands * 8, cudaMemcpyHostToDevice)) != cudaSuccess) {
+            s->ff.release();
             return cuda_fail(ctx, e, "bpm upload");
+        }
     }
     d.pos = s->pos.p;
     d.geo = s->geo.p;
@@ -1005,12 +1008,13 @@ static int bpm_enqueue(acum_ctx* ctx, BBDev& d, int aa_mode, const float* seed_s
             return cuda_fail(ctx, e, "bpm configure");
         configured = true;
     }
-    static int per_sm = 0;
-    if (per_sm == 0 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bb_obs_kernel, kBpmThreads, kObsSmem) !=
-                            cudaSuccess ||
-                        per_sm < 1))
-        per_sm = 1;
-    const int slots = per_sm * ctx->num_sms;
+    if (s->per_sm == 0 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s->per_sm, bb_obs_kernel, kBpmThreads,
+                                                                         kObsSmem) != cudaSuccess ||
+                           s->per_sm < 1)) {
+        (void)cudaGetLastError();
+        s->per_sm = 1;
+    }
+    const int slots = s->per_sm * ctx->num_sms;
     int split = 1;
     double best = 1e30;
     const int maxs = (int)std::max<long long>(1, std::min<long long>((8 * slots + oblocks - 1) / oblocks,
