@@ -65,7 +65,7 @@ using namespace acum;
 
 // ---------------------------------------------------------------- lifecycle
 
-void acum_ctx::release_all()
+void acum_ctx::release_work()
 {
     d_raw.release();
     d_raw_alt.release();
@@ -84,10 +84,17 @@ void acum_ctx::release_all()
     d_acc.release();
     d_out.release();
     d_rec32.release();
-    d_err.release();
     for (auto& b : d_per) b.release();
     acum::release_bpm_state(this);
     acum::release_adj_state(this);
+    have_deck = false;
+    invalidate();
+}
+
+void acum_ctx::release_all()
+{
+    release_work();
+    d_err.release();
 }
 
 extern "C" int acum_version(void) { return 1; }
@@ -790,13 +797,52 @@ extern "C" int acum_host_free(void* p)
 
 namespace acum {
 
+namespace {
+
+// Id of the current CUDA context, which no other context of the process ever has: device memory,
+// streams and page-locked memory belong to a context, and a new one (after cudaDeviceReset) may
+// hold other things at their addresses.
+bool context_id(unsigned long long* id)
+{
+    using GetId = int (*)(void*, unsigned long long*);
+    static const GetId get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<GetId>(f);
+    }();
+    if (!get) return false;
+    if (get(nullptr, id) == 0) return true;
+    // none is current yet, or it has gone: cudaFree makes the device's current
+    return cudaFree(nullptr) == cudaSuccess && get(nullptr, id) == 0;
+}
+
+// by kind and context, until the process ends (recursive: creating one may give back others)
+struct Dropins {
+    std::recursive_mutex mu;
+    std::map<std::pair<int, unsigned long long>, Dropin*> all;
+};
+Dropins& dropins()
+{
+    static Dropins* d = new Dropins();
+    return *d;
+}
+
+}  // namespace
+
 Dropin* dropin_for(int dev, int kind)
 {
-    static std::mutex mu;
-    static std::map<int, Dropin*> all[kDropinKinds];  // until the process ends
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = all[kind].find(dev);
-    if (it != all[kind].end()) return it->second;
+    unsigned long long id = 0;
+    if (!context_id(&id)) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    Dropins& r = dropins();
+    std::lock_guard<std::recursive_mutex> lk(r.mu);
+    auto it = r.all.find({kind, id});
+    if (it != r.all.end()) return it->second;
     std::unique_ptr<Dropin> d(new Dropin());
     if (acum_create(&d->c, dev) != ACUM_OK) return nullptr;
     void* p = nullptr;
@@ -808,7 +854,25 @@ Dropin* dropin_for(int dev, int kind)
     }
     d->facts = static_cast<DropinFacts*>(p);
     d->err = reinterpret_cast<DeviceErr*>(d->facts + 1);
-    return all[kind][dev] = d.release();
+    return r.all[{kind, id}] = d.release();
+}
+
+bool give_back_workspaces()
+{
+    unsigned long long id = 0;
+    if (!context_id(&id)) return false;
+    Dropins& r = dropins();
+    std::lock_guard<std::recursive_mutex> lk(r.mu);
+    bool any = false;
+    for (auto& e : r.all) {
+        Dropin* d = e.second;
+        // busy: possibly this thread's own call
+        if (e.first.second != id || d->busy || !d->mu.try_lock()) continue;
+        d->c->release_work();
+        d->mu.unlock();
+        any = true;
+    }
+    return any;
 }
 
 }  // namespace acum
@@ -830,7 +894,7 @@ int find_pth(const S* rObs, const S* tObs, S* pT, S* pL, S* pA, const S* Xham, c
     if (ce != cudaSuccess) return cuda_fail(nullptr, ce, "cudaGetDevice");
     Dropin* dr = dropin_for(dev, kDropinTonal);
     if (!dr) return fail(nullptr, ACUM_ERR_CUDA, "findPressureTimeHistory: cannot create a context");
-    std::lock_guard<std::mutex> lock(dr->mu);
+    DropinLock lock(dr);
     acum_ctx* c = dr->c;
     cudaStream_t st = stream_v ? (cudaStream_t)stream_v : (cudaStream_t)0;
     // the small per-surface arrays and the bin grid live in device memory, as the reference
@@ -957,7 +1021,7 @@ extern "C" int acum_preprocess_imper(float* Xham, float* Nham, float* Vham, floa
     if (ce != cudaSuccess) return cuda_fail(nullptr, ce, "cudaGetDevice");
     Dropin* dr = dropin_for(dev, kDropinTonal);
     if (!dr) return fail(nullptr, ACUM_ERR_CUDA, "preprocess_imper: cannot create a context");
-    std::lock_guard<std::mutex> lock(dr->mu);
+    DropinLock lock(dr);
     acum_ctx* c = dr->c;
     InFlight flight(c->stream);
     // surface rows from the AoS arrays (what read_surf stored, io.cu:318)
@@ -1179,7 +1243,7 @@ int preprocess_per_t(S* Xham, S* Nham, S* Vham, S* Uham, S* PRham, int nSurf, co
     if (ce != cudaSuccess) return cuda_fail(nullptr, ce, "cudaGetDevice");
     Dropin* dr = dropin_for(dev, kDropinTonal);
     if (!dr) return fail(nullptr, ACUM_ERR_CUDA, "preprocess_per: cannot create a context");
-    std::lock_guard<std::mutex> lock(dr->mu);
+    DropinLock lock(dr);
     acum_ctx* c = dr->c;
     cudaStream_t st = c->stream;
     S* host[5] = {Xham, Nham, Vham, Uham, PRham};

@@ -371,6 +371,8 @@ extern "C" int acum_batch_add(acum_batch* b, const acum_inputs* in, int nobs, co
     const double sums = (double)nobs * T * 8 * 3;
     size_t free_b = 0, total_b = 0;
     BK(b, cudaMemGetInfo(&free_b, &total_b));
+    if (rows + recs + sums + (double)(1ull << 30) > (double)free_b && give_back_workspaces())
+        BK(b, cudaMemGetInfo(&free_b, &total_b));
     if (rows + recs + sums + (double)(1ull << 30) > (double)free_b)
         return bfail(b, ACUM_ERR_NOMEM, "acum_batch_add: not enough free device memory for this case");
     acum_ctx* c = nullptr;

@@ -1316,7 +1316,7 @@ extern "C" int acum_find_bb_noise(int nSurf_BB, int nObs, int nTime, float dTau,
     if (e != cudaSuccess) return cuda_fail(nullptr, e, "cudaGetDevice");
     Dropin* dr = dropin_for(dev, kDropinBroadband);
     if (!dr) return fail(nullptr, ACUM_ERR_CUDA, "findBBnoise: cannot create a context");
-    std::lock_guard<std::mutex> lock(dr->mu);
+    DropinLock lock(dr);
     acum_ctx* c = dr->c;
     DeviceGuard g(dev);
     BpmState* s = state(c);

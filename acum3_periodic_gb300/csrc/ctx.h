@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -12,6 +13,10 @@
 #include "deck.h"
 
 namespace acum {
+
+// Frees the workspaces that idle reference-shaped calls keep (Dropin) in the current context;
+// whether there were any.
+bool give_back_workspaces();
 
 template <typename T>
 struct DBuf {
@@ -23,7 +28,12 @@ struct DBuf {
         if (p) cudaFree(p);
         p = nullptr;
         n = 0;
-        cudaError_t e = cudaMalloc(&p, std::max<size_t>(want, 1) * sizeof(T));
+        const size_t bytes = std::max<size_t>(want, 1) * sizeof(T);
+        cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation && give_back_workspaces()) {
+            (void)cudaGetLastError();
+            e = cudaMalloc(&p, bytes);
+        }
         if (e == cudaSuccess) n = want;
         else p = nullptr;
         return e;
@@ -91,15 +101,32 @@ int cuda_fail(struct ::acum_ctx* ctx, cudaError_t e, const char* what);
 void derive(const acum_inputs& in, Derived& d);
 void release_bpm_state(struct ::acum_ctx* ctx);
 
-// The workspaces of the reference-shaped calls on one device, kept from call to call (their
-// buffers are scratch; nothing of a call's data is used by the next).  `mu` is held for the
-// whole call, every way out of which waits for its stream (InFlight): one call at a time per
-// device and kind.
+// The workspaces of the reference-shaped calls in one CUDA context, kept from call to call
+// (their buffers are scratch; nothing of a call's data is used by the next).  DropinLock holds
+// `mu` for the whole call, every way out of which waits for its stream (InFlight): one call at
+// a time per context and kind.  They are given back when an allocation of this library fails
+// (give_back_workspaces); a context that has gone (cudaDeviceReset) took its own with it.
 struct Dropin {
     std::mutex mu;
+    std::atomic<bool> busy{false};  // mu is held by a call
     struct ::acum_ctx* c = nullptr;
     DropinFacts* facts = nullptr;  // page-locked, written by the device
     DeviceErr* err = nullptr;      // page-locked
+};
+struct DropinLock {
+    Dropin* d;
+    explicit DropinLock(Dropin* dropin) : d(dropin)
+    {
+        d->mu.lock();
+        d->busy = true;
+    }
+    ~DropinLock()
+    {
+        d->busy = false;
+        d->mu.unlock();
+    }
+    DropinLock(const DropinLock&) = delete;
+    DropinLock& operator=(const DropinLock&) = delete;
 };
 enum { kDropinTonal = 0, kDropinBroadband = 1, kDropinKinds };
 Dropin* dropin_for(int device, int kind);  // null: cannot create a context
@@ -183,6 +210,7 @@ struct acum_ctx {
         launches = 0;
         prep_timed = tonal_timed = bpm_timed = adj_timed = call_timed = false;
     }
+    void release_work();  // every device buffer but the error word
     void release_all();
     int upload_deck_common(const acum_inputs& inp, int nob, const float* obs_file, int ns, const int* ne);
     int ensure_prep(bool need64, bool need32, bool need_fields);

@@ -337,7 +337,9 @@ int acum_preprocess_per_device(void* Xham, void* Nham, void* Vham, void* Uham, v
 /* Replaces findBBnoise (bb_core.cu:11) as called at main.cu:150: the same 39 arguments,
  * host pointers, FP32 storage; BBspl [nObs][nf2][7] and BBoaspl [nObs] are updated as the
  * reference does (they arrive seeded, normally with -100 dB).  Computes on the GPU with
- * aa_mode 0 (see acum_bpm). */
+ * aa_mode 0 (see acum_bpm).  Calls from several threads run one at a time on a device.  Up to
+ * 512 MiB of device memory stays with the library for the next call, until an allocation of
+ * the library fails or the device is reset. */
 int acum_find_bb_noise(int nSurf_BB, int nObs, int nTime, float dTau, const float* span, const float* omega,
                        const int* ccw, const float* psi_offset, const int* trip, const float* rotate,
                        const float* translate, const int* xsPtr, const int* dsPtr, const int* nsect,
