@@ -52,7 +52,7 @@ struct AdjDev {
     double* cot;      // [E][T][kCot] FP64
 };
 
-// reciprocal and square root: within 0.51 ulp in FP64, the fast hardware forms in FP32 (the
+// reciprocal and square root: IEEE in FP64, the fast hardware forms in FP32 (the
 // FP32 adjoint is compared with the FP64 one, not with the reference)
 __device__ __forceinline__ double rcp_(double x) { return rcp_d(x); }
 __device__ __forceinline__ float rcp_(float x) { return rcp_ftz(x); }

@@ -1,7 +1,8 @@
 // probe.cu -- measures the FP32 and FP64 FMA throughput of the device (the CUDA-core
 // peaks the tonal kernels are compute-bound against), with CUDA events; a self-test of
 // the bounded barrier wait that every pipelined kernel uses; and a self-test of the
-// shared-memory to tensor-memory copy and the tensor-memory loads of the record stages.
+// shared-memory to tensor-memory copy and the tensor-memory loads of the record stages; a
+// self-test of the FP64 operations that the kernels form in integers.
 #include <cuda_runtime.h>
 
 #include "acum_internal.h"
@@ -127,7 +128,52 @@ __global__ void __launch_bounds__(512, 1) tmem_selftest_kernel(int* mismatches, 
     if (warp == 0) acum::tmem_dealloc(tbase, 64);
 }
 
+// The operations of ptx.h and the FP64 instructions in whose place they stand, one operand pair
+// a thread.
+__global__ void __launch_bounds__(256) arith_selftest_kernel(int which, int n, const double* a, const double* b,
+                                                             double* got, double* want)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double x = a[i], y = b[i];
+    double g, w;
+    switch (which) {
+    case 0: g = acum::rcp_d(x); w = 1.0 / x; break;
+    case 1: g = acum::sqrt_d(x); w = sqrt(x); break;
+    case 2: g = acum::mul_d(x, y); w = __dmul_rn(x, y); break;
+    case 3: g = (double)acum::floor_d(x); w = (double)(int)floor(x); break;
+    case 4: g = acum::int_d((int)x); w = (double)(int)x; break;
+    case 5: g = acum::widen_d((float)x); w = (double)(float)x; break;
+    default: g = (double)acum::narrow_d(x); w = (double)(float)x; break;
+    }
+    got[i] = g;
+    want[i] = w;
+}
+
 }  // namespace
+
+extern "C" int acum_selftest_arith(int device, int which, int n, const double* a, const double* b, double* got,
+                                   double* want)
+{
+    if (!a || !b || !got || !want || n <= 0 || which < 0 || which > 6) return ACUM_ERR_INVALID;
+    int prev = 0;
+    cudaGetDevice(&prev);
+    if (cudaSetDevice(device) != cudaSuccess) return ACUM_ERR_CUDA;
+    const size_t bytes = (size_t)n * sizeof(double);
+    double* d = nullptr;  // a, b, got, want
+    cudaError_t e = cudaMalloc(&d, 4 * bytes);
+    if (e == cudaSuccess) e = cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        arith_selftest_kernel<<<(unsigned)(((size_t)n + 255) / 256), 256>>>(which, n, d, d + n, d + 2 * (size_t)n, d + 3 * (size_t)n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(got, d + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(want, d + 3 * (size_t)n, bytes, cudaMemcpyDeviceToHost);
+    if (d) cudaFree(d);
+    cudaSetDevice(prev);
+    return e == cudaSuccess ? ACUM_OK : ACUM_ERR_CUDA;
+}
 
 extern "C" int acum_selftest_tmem(int device, int* mismatches, unsigned* readback)
 {

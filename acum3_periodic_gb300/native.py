@@ -75,6 +75,7 @@ SIGNATURES = {
     "acum_tonal_from_host_async": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
     "acum_selftest_wait": (C.c_int, [C.c_int, C.c_double, C.c_int, _IP, _DP]),
     "acum_selftest_tmem": (C.c_int, [C.c_int, _IP, C.c_void_p]),
+    "acum_selftest_arith": (C.c_int, [C.c_int, C.c_int, C.c_int, _DP, _DP, _DP, _DP]),
     "acum_read_deck_sizes": (C.c_int, [C.c_char_p, C.POINTER(C.c_longlong)]),
     "acum_write_surface_cache": (C.c_int, [C.c_char_p]),
     "acum_last_plan": (C.c_int, [C.c_void_p, _IP]),
@@ -468,6 +469,17 @@ def selftest_tmem(device: int = 0):
     if rc != 0:
         raise AcumError(rc, "acum_selftest_tmem failed")
     return mis.value, rb
+
+
+def selftest_arith(which: int, a, b=None, device: int = 0):
+    """(got, want) of the operation `which` of acum_selftest_arith on the operands a (and b)."""
+    a = np.ascontiguousarray(a, np.float64)
+    b = a if b is None else np.ascontiguousarray(b, np.float64)
+    got, want = np.empty_like(a), np.empty_like(a)
+    rc = lib().acum_selftest_arith(device, which, a.size, _p(a), _p(b), _p(got), _p(want))
+    if rc != 0:
+        raise AcumError(rc, "acum_selftest_arith failed")
+    return got, want
 
 
 def preprocess_per(ne, X, N, V, U, PR, dTau, a0, rhoRef, Mref, CFDscale, periodic=1, lowpass=0,

@@ -244,6 +244,11 @@ int acum_selftest_wait(int device, double limit_s, int arrive, int* timed_out, d
  * complete within the bounded wait); readback (optional, 4 x 32 x 40 words) = what warps
  * 0-3 read, lane by lane. */
 int acum_selftest_tmem(int device, int* mismatches, unsigned* readback);
+/* Self-test of the FP64 operations that the kernels form in integers, beside the FP64
+ * instruction of each, over n host operands a (and b): which = 0: 1 / a, 1: sqrt(a), 2: a b,
+ * 3: floor(a) as an int, 4: int a as a double, 5: float a as a double, 6: a as a float (3 to 6
+ * as doubles).  got and want hold the same values (NaN for NaN) where a device passes. */
+int acum_selftest_arith(int device, int which, int n, const double* a, const double* b, double* got, double* want);
 
 /* Measured FMA throughput of `device` in TFLOP/s: which = 0 FP32, 1 FP64 (a short
  * FMA-chain kernel timed with CUDA events; the CUDA-core peaks of the roofline). */
