@@ -48,6 +48,7 @@ struct AdjDev {
     const void* obs;  // [O][3]
     const void* g;    // [O][T]
     double a0, alpha, ialpha, vx, vy, vz, dTau, oM, dPsi, kb;
+    F64Time time;
     unsigned tmod;    // ceil(2^32 / T)
     double* cot;      // [E][T][kCot] FP64
 };
@@ -222,11 +223,12 @@ __global__ void __launch_bounds__(128, 4) adjoint_kernel(AdjDev p)
     const double* obs = reinterpret_cast<const double*>(p.obs);
     const double* gg = reinterpret_cast<const double*>(p.g);
     const OnWind<double> v = on_wind(f, p);
-    const double kb = p.kb, uT = (double)tau * (p.dTau * kb);
+    // observer times in bins, from the bin of this window's lane 0 (tonal.cu: F64Time)
+    const double kb = p.time.kb, kbl = p.time.kbl, uT = (double)lane + (double)tau * p.time.eps;
     for (int o = 0; o < p.O; ++o) {
         const Fwd<double> a = forward<F>(f, obs[3 * o], obs[3 * o + 1], obs[3 * o + 2], p);
         // observer time in bins and its floor, as the forward forms them
-        const double u = fma(kb, a.tr, uT);
+        const double u = fma(kb, a.tr, fma(kbl, a.tr, uT));
         const int nb = floor_d(u);
         const double pc = mul_d(a.w2, a.S);
         const double up = __shfl_up_sync(0xffffffffu, u, 1);
@@ -243,7 +245,8 @@ __global__ void __launch_bounds__(128, 4) adjoint_kernel(AdjDev p)
         // the time derivatives are -(dp / du) times those sums
         double wgt = mul_d(int_d(n0) - up, inv);
         const double* grow = gg + (size_t)o * p.T;
-        int idx = n0 >= 0 && n0 < (1 << 24) ? wrap_T(n0, p.T, p.tmod) : ((n0 % p.T) + p.T) % p.T;
+        const int n = tau - lane + n0;
+        int idx = n >= 0 && n < (1 << 24) ? wrap_T(n, p.T, p.tmod) : ((n % p.T) + p.T) % p.T;
         double sg = cnt > 0 ? grow[idx] : 0.0, rp = mul_d(sg, wgt);
         while (--cnt > 0) {
             if (++idx == p.T) idx = 0;
@@ -772,6 +775,7 @@ extern "C" int acum_tonal_adjoint(acum_ctx* ctx, int precision, const double* dJ
     p.oM = ctx->der.oM;
     p.dPsi = ctx->der.dPsi;
     p.kb = p.oM / p.dPsi;
+    p.time = f64_time(p.oM, p.dPsi, p.dTau);
     p.tmod = (unsigned)((0x100000000ull + (unsigned long long)ctx->T - 1) / (unsigned long long)ctx->T);
     CKA(s->cot.ensure((size_t)E * T * kCot));
     p.cot = s->cot.p;
