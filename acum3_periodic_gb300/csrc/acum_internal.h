@@ -273,6 +273,40 @@ struct PrepArgs {
 // with rec32: also the anchors of `job`
 cudaError_t launch_prep(const PrepArgs& a, const AnchorJob& job, cudaStream_t s);
 
+// Pairs of floats as unevaluated sums x + y (T. J. Dekker, Numer. Math. 18, 1971; TwoSum: D. E.
+// Knuth, The Art of Computer Programming 2, 4.2.2): the product and the sum of two floats, exactly.
+__host__ __device__ __forceinline__ float2 prod2(float a, float b)
+{
+    const float p = a * b;
+    return make_float2(p, fmaf(a, b, -p));
+}
+__host__ __device__ __forceinline__ float2 sum2(float a, float b)
+{
+    const float s = a + b, t = s - a;
+    return make_float2(s, (a - (s - t)) + (b - t));
+}
+// the product of two pairs, to about 2^-46
+__host__ __device__ __forceinline__ float2 mul_pair(float2 a, float2 b)
+{
+    const float p = a.x * b.x;
+    return make_float2(p, fmaf(a.x, b.x, -p) + fmaf(a.x, b.y, a.y * b.x));
+}
+// a b + c d and a.b as pairs, to about 2^-48 of the result, or 2^-70 of the largest term where the
+// terms cancel: the rounding errors of the products and sums are summed with theirs in turn
+__host__ __device__ __forceinline__ float2 dot2(float a, float b, float c, float d)
+{
+    const float2 p = prod2(a, b), q = prod2(c, d), s = sum2(p.x, q.x);
+    const float2 l = sum2(p.y, q.y), m = sum2(s.y, l.x), h = sum2(s.x, m.x);
+    return sum2(h.x, h.y + (l.y + m.y));
+}
+__host__ __device__ __forceinline__ float2 dot3(const float* a, const float* b)
+{
+    const float2 p = prod2(a[0], b[0]), q = prod2(a[1], b[1]), r = prod2(a[2], b[2]);
+    const float2 s = sum2(p.x, q.x), t = sum2(s.x, r.x);
+    const float2 l = sum2(s.y, t.y), m = sum2(p.y, q.y), n = sum2(l.x, m.x), o = sum2(n.x, r.y), h = sum2(t.x, o.x);
+    return sum2(h.x, h.y + ((l.y + m.y) + (n.y + o.y)));
+}
+
 // records straight from reference-layout AoS arrays (for the drop-in entry points)
 struct AosArgs {
     const void* X;  // float or double, AoS as variables.cu:54
