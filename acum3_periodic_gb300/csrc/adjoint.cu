@@ -443,6 +443,7 @@ __global__ void adj_seed_kernel(const double* __restrict__ acc, int O, int T, do
 struct ChainDev {
     const double* cot;     // [E][T][kCot]
     const double* fields;  // [E][T][18] from the preprocessing
+    const double* cub;     // [E][5] from the preprocessing: make_periodic's cubics
     int E, T, periodic, lowpass;
     double a0, rho, pscale, cfd, dTau;
     double gauss[13];
@@ -602,23 +603,9 @@ __global__ void __launch_bounds__(256) adjoint_chain_kernel(ChainDev c)
         double* B = bVd + T;
         const int s = c.e_surf[e], j = c.e_local[e], Es = c.e_count[s];
         const float* base = c.raw + c.raw_off[s];
-        for (int t = threadIdx.x; t < T; t += blockDim.x) Pm[t] = (double)base[((size_t)t * Es + j) * 8 + 3] * c.pscale;
-        __syncthreads();
-        {
-            const double p0 = Pm[0], p1 = Pm[1], pm = Pm[T - 2], pn = Pm[T - 1];
-            const double g0 = p0 - (p1 - p0);
-            const double k2 = pn, k1 = g0, s2 = pn - pm, s1 = p0 - g0;
-            const int xm = T;
-            const double dd = k1, cc = s1 - s2;
-            const double bb = -2.0 * (s1 - s2) / xm - 3.0 * (k1 - k2) / xm / xm;
-            const double aa = -bb / xm - (s1 - s2) / xm / xm - (k1 - k2) / xm / xm / xm;
-            __syncthreads();
-            for (int t = threadIdx.x; t < T; t += blockDim.x) {
-                const int i = t + 1;
-                const double cub = aa * i * i * i + bb * i * i + cc * i + dd;
-                Pm[t] = Pm[t] - (cub - k2);
-            }
-        }
+        const double* cub = c.cub + (size_t)e * 5;
+        for (int t = threadIdx.x; t < T; t += blockDim.x)
+            Pm[t] = periodic_pressure(base[((size_t)t * Es + j) * 8 + 3], c.pscale, cub, t);
         __syncthreads();
         for (int t = threadIdx.x; t < T; t += blockDim.x) {
             const double l = Pm[t == 0 ? T - 1 : t - 1], m = Pm[t], r = Pm[t == T - 1 ? 0 : t + 1];
@@ -804,6 +791,7 @@ extern "C" int acum_tonal_adjoint(acum_ctx* ctx, int precision, const double* dJ
     ChainDev c;
     c.cot = s->cot.p;
     c.fields = ctx->d_fields.p;
+    c.cub = ctx->d_cub.p;
     c.E = (int)E;
     c.T = T;
     c.periodic = ctx->in.periodic;
