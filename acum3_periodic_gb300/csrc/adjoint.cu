@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(256) adjoint_chain_kernel(ChainDev c)
     double* tmp = bPd + T;      // [3][T]
     const int e = blockIdx.x;
     const double D1 = 1.0 / (4.0 * M_PI * c.a0), ia2 = 1.0 / (c.a0 * c.a0);
-    const double i2dt = 1.0 / (2.0 * c.dTau);  // as the preprocessing: products, not quotients
+    const double two_dt = 2.0 * c.dTau;
     // local chain at each step
     for (int t = threadIdx.x; t < T; t += blockDim.x) {
         const double* k = c.cot + ((size_t)e * T + t) * kCot;
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(256) adjoint_chain_kernel(ChainDev c)
     // transposes of the periodic central difference: D^T v[k] = (v[k-1] - v[k+1]) / (2 dt)
     auto DT = [&](const double* v, int k) {
         const int km = k == 0 ? T - 1 : k - 1, kp = k == T - 1 ? 0 : k + 1;
-        return (v[km] - v[kp]) * i2dt;
+        return (v[km] - v[kp]) / two_dt;
     };
     // Vd = D V: bV += D^T bVd
     for (int t = threadIdx.x; t < T; t += blockDim.x)
@@ -584,8 +584,8 @@ __global__ void __launch_bounds__(256) adjoint_chain_kernel(ChainDev c)
             };
             // u[t] appears in du[t-1] (+1/(2dt)) and du[t+1] (-1/(2dt)) for interior rows
             double acc = bP[t];
-            if (t - 1 >= 1 && t - 1 <= T - 2) acc += w(t - 1) * i2dt;
-            if (t + 1 >= 1 && t + 1 <= T - 2) acc -= w(t + 1) * i2dt;
+            if (t - 1 >= 1 && t - 1 <= T - 2) acc += w(t - 1) / two_dt;
+            if (t + 1 >= 1 && t + 1 <= T - 2) acc -= w(t + 1) / two_dt;
             tmp[t] = acc;
         }
     }
