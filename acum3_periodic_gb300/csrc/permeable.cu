@@ -41,8 +41,11 @@ constexpr int kPerRows = 6;
 // smaller blocks put more elements on an SM (20000 elements x 100 steps, filtered, float:
 // 2.23 ms in blocks of 256, 1.24 in blocks of 64; 3000 x 60 349 -> 198 us); long ones form
 // fewer products in longer runs (8192 x 1440 6.60 ms with runs of 17, 6.30 with 23; 20000 x 100
-// with runs of 13 1.76, of 9 1.37).
-constexpr int kSmallT = 160, kMediumT = 512, kShortRun = 17, kLongRun = 23;
+// with runs of 13 1.76, of 9 1.37).  Past the period at which a block still holds two series' long
+// runs it filters one at a time either way, and short runs are the shorter ones (2000 elements x
+// 3000 steps, float and double, 4.98 and 4.89 ms with runs of 23, 4.27 and 4.18 with 17; 1666 x 3600
+// 4.18 and 4.19, 3.97 and 3.98; 1464 x 4096 4.00 and 3.92, 4.02 and 3.95).
+constexpr int kSmallT = 160, kMediumT = 512, kShortRun = 17, kLongRun = 23, kLongT = kPerThreads / 2 * kLongRun;
 
 template <typename S>
 struct PerPtrs {
@@ -345,10 +348,10 @@ cudaError_t launch_per_s(void* X, void* N, void* V, void* U, void* PR, const Per
     const PerPtrs<S> p{(S*)X, (S*)N, (S*)V, (S*)U, (S*)PR};
     const int threads = a.T <= kSmallT ? 64 : a.T <= kMediumT ? 128 : kPerThreads;
     if (a.lowpass != 1) return launch_per_t<S, Q, 0>(p, a, threads, s);
-    static_assert(kSmallT <= 64 * kShortRun && kMediumT <= 128 * kShortRun && kMaxPerSteps <= kPerThreads * kLongRun,
+    static_assert(kSmallT <= 64 * kShortRun && kMediumT <= 128 * kShortRun && kMaxPerSteps <= kPerThreads * kShortRun,
                   "a series' runs fit in a block");
-    return a.T <= kMediumT ? launch_per_t<S, Q, kShortRun>(p, a, threads, s)
-                         : launch_per_t<S, Q, kLongRun>(p, a, threads, s);
+    return a.T <= kMediumT || a.T > kLongT ? launch_per_t<S, Q, kShortRun>(p, a, threads, s)
+                                           : launch_per_t<S, Q, kLongRun>(p, a, threads, s);
 }
 
 // The rows of a permeable deck as read_surf leaves them (io.cu:263-293): each 12-column

@@ -114,3 +114,10 @@ def test_many_surfaces_and_odd_starts():
                     np.testing.assert_array_equal(got[s0:s0 + n * T * w], b[e0:e0 + n].astype(dt).reshape(-1), err_msg=nm)
                     seen[s0:s0 + n * T * w] = True
                 assert (got[~seen] == 7.0).all(), nm
+
+
+@pytest.mark.parametrize("ntime", [2944, 2945, 3000, 4080, 4096])
+@pytest.mark.parametrize("periodic,lowpass", [(1, 1), (0, 1), (0, 0)])
+def test_long_periods(ntime, periodic, lowpass):
+    """Both sides of the period from which a block filters one series at a time, in short runs."""
+    test_periods(ntime, periodic, lowpass)
