@@ -543,7 +543,6 @@ int acum_ctx::run_tonal(int precision, double* d_pT, double* d_pL, double* d_pA)
     r.g.oM = der.oM;
     r.g.dPsi = der.dPsi;
     r.g.dTau = der.dTau;
-    r.g.lpi = T * der.dPsi;
     for (int c = 0; c < 3; ++c) r.g.vinf[c] = der.vinf[c];
     r.g.obs_rmin = obs_rmin;
     r.precision = precision;
@@ -922,7 +921,6 @@ int find_pth(const S* rObs, const S* tObs, S* pT, S* pL, S* pA, const S* Xham, c
     r.g.oM = oM;
     r.g.dPsi = dPsi;
     r.g.dTau = dTau;
-    r.g.lpi = nTime * dPsi;
     for (int q = 0; q < 3; ++q) r.g.vinf[q] = facts.vinf[q];
     r.g.obs_rmin = facts.obs_rmin;
     r.precision = f64 ? ACUM_PLAIN_FP64 : ACUM_MIXED;

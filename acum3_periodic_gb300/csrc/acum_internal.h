@@ -198,7 +198,7 @@ struct DeviceErr {
 
 struct TonalGeom {
     int E, Epad, T, nW, O;
-    double a0, rho, oM, dPsi, dTau, lpi;  // dPsi in radians
+    double a0, rho, oM, dPsi, dTau;  // dPsi in radians
     double vinf[3];
     double obs_rmin;  // smallest observer distance from the origin (of the FP32 positions; < 0 unknown)
 };
@@ -412,7 +412,7 @@ struct KParams {
     unsigned tmod;  // ceil(2^32 / T): bin index modulo T by multiply-high
     // FP64 constants
     F64Time time;
-    double a0, alpha, ialpha, vx, vy, vz, dTau, oM, dPsi, lpi;
+    double alpha, ialpha, vx, vy, vz, dPsi;
     int W, NS, chunk, nchunk, obs_tiles, flush_groups, tile_group;
     double* acc;
     DeviceErr* err;

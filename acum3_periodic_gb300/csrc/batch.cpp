@@ -103,7 +103,6 @@ TonalRun case_run(const acum_batch* b, const acum_ctx* c, double* acc)
     r.g.oM = c->der.oM;
     r.g.dPsi = c->der.dPsi;
     r.g.dTau = c->der.dTau;
-    r.g.lpi = c->T * c->der.dPsi;
     for (int k = 0; k < 3; ++k) r.g.vinf[k] = c->der.vinf[k];
     r.g.obs_rmin = c->obs_rmin;
     r.precision = ACUM_MIXED;

@@ -42,7 +42,7 @@
 
 namespace acum {
 
-constexpr int kMaxAoa = 64;
+constexpr int kMaxAoa = 64;  // tables with more AoA entries are refused
 constexpr int kSc = 32;    // spectral scalars per (section, step)
 constexpr int kGeo = 16;   // geometry record per (section, step)
 constexpr int kAmp = 8;    // amplitudes per (section, step, band)

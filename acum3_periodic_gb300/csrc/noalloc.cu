@@ -155,7 +155,6 @@ extern "C" int acum_find_pressure_time_history_noalloc(const float* rObs, const 
     r.g.oM = oM;
     r.g.dPsi = dPsi;
     r.g.dTau = dTau;
-    r.g.lpi = nTime * (double)dPsi;
     const double* vi = facts.vinf;
     for (int q = 0; q < 3; ++q) r.g.vinf[q] = vi[q];
     r.g.obs_rmin = obs_rmin;
