@@ -198,13 +198,13 @@ __device__ __forceinline__ void close(const R* f, R* acc)
         acc[i] -= acc[kCot] * f[4 + i] - acc[7] * f[8 + i] + acc[kCot + 1] * f[12 + i] - acc[14] * f[16 + i];
 }
 
-// Bound by the FP64 pipe: about 72 of its instructions an evaluation in flight without a y
+// Bound by the FP64 pipe: about 70 of its instructions an evaluation in flight without a y
 // component, from 203 with IEEE quotients and root, the projections scaled by 1/r, the retarded
 // time's chain of derivatives written out, the observer time in radians, the position's share of
 // every projection formed for each observer, and products, quotients and roots on the pipe
-// (workload 3, 4800 elements, 360 steps, 256 observers: 163.8 -> 59.9 ms, of which 45 by taking
+// (workload 3, 4800 elements, 360 steps, 256 observers: 163.8 -> 62.0 ms, of which 45 by taking
 // products, quotients and the root to the integers; in FP32, the same reverse pass, 5.10 -> 3.73
-// ms; with 64 observers 40.9 -> 15.1 ms).
+// ms; with 64 observers 40.9 -> 15.6 ms).
 template <Wind F>
 __global__ void __launch_bounds__(128, 4) adjoint_kernel(AdjDev p)
 {

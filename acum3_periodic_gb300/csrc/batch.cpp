@@ -199,7 +199,9 @@ int ring_cases(acum_batch* b)
 // chunks, so that every FP32 sum is the same one: less padding in a case's last tile and a
 // shorter last round.  Launches in us, 32 -> 16: 24 cases of 1600 elements x 360 steps x 96
 // observers 1968 -> 1895, 20 of 2500 x 360 x 72 2384 -> 2054, 40 of 3000 x 480 x 16 2495 ->
-// 1312, 40 of 3000 x 480 x 128 10630 -> 10580, 10 of 800 x 200 x 20 113 -> 117.
+// 1312, 40 of 3000 x 480 x 128 10630 -> 10580, 10 of 800 x 200 x 20 113 -> 117.  Launches of less
+// than one wave lose up to 7 % (5 us); over 431 batches 1.22 times as fast in geometric mean
+// (profiles/ring_shapes.md).
 void default_shape(acum_batch* b)
 {
     b->W = 32;
