@@ -1248,7 +1248,7 @@ int preprocess_per_t(S* Xham, S* Nham, S* Vham, S* Uham, S* PRham, int nSurf, co
     PerBuffers b;
     InFlight flight(st);
     for (int q = 0; q < 5; ++q) {
-        CK(nullptr, cudaMalloc(&b.d[q], (size_t)L.extent[q] * sizeof(S)));
+        CK(nullptr, device_alloc(&b.d[q], (size_t)L.extent[q] * sizeof(S)));
         CK(nullptr, cudaMemcpyAsync(b.d[q], host[q], (size_t)L.extent[q] * sizeof(S), cudaMemcpyHostToDevice, st));
     }
     rc = per_enqueue(b.d, sizeof(S) == 8, L, nTime, dTau, a0, rhoRef, Mref, CFDscale, periodic, lowpass, st);

@@ -18,6 +18,17 @@ namespace acum {
 // whether there were any.
 bool give_back_workspaces();
 
+// cudaMalloc, once more where those can be given back
+inline cudaError_t device_alloc(void** p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && give_back_workspaces()) {
+        (void)cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
 template <typename T>
 struct DBuf {
     T* p = nullptr;
@@ -28,12 +39,7 @@ struct DBuf {
         if (p) cudaFree(p);
         p = nullptr;
         n = 0;
-        const size_t bytes = std::max<size_t>(want, 1) * sizeof(T);
-        cudaError_t e = cudaMalloc(&p, bytes);
-        if (e == cudaErrorMemoryAllocation && give_back_workspaces()) {
-            (void)cudaGetLastError();
-            e = cudaMalloc(&p, bytes);
-        }
+        cudaError_t e = device_alloc(reinterpret_cast<void**>(&p), std::max<size_t>(want, 1) * sizeof(T));
         if (e == cudaSuccess) n = want;
         else p = nullptr;
         return e;
